@@ -6,14 +6,15 @@ missing or does not load -- there is no CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
+import importlib.util
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libnuvec_cuda.so"
 
-try:
-    from . import _native as native  # the operators' host path (csrc/native.cpp)
-except ImportError:  # not built yet: the package imports (its build module has to), opening a device does not work
-    native = None
+if importlib.util.find_spec(f"{__package__}._native") is None:
+    raise ImportError(f"{__package__}._native is missing: build it with `python -m nuvec_b200.build`")
+native = importlib.import_module(f"{__package__}._native")  # the operators' host path (csrc/native.cpp)
 
 OK = 0
 ERR_INVALID_ARGUMENT, ERR_UNSUPPORTED, ERR_OUT_OF_MEMORY, ERR_NO_DEVICE, ERR_DRIVER, ERR_COMM = -1, -2, -3, -4, -5, -6
@@ -150,8 +151,6 @@ def lib():
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(handle, name)  # AttributeError if the export is missing
             fn.restype, fn.argtypes = res, args
-        if native is None:
-            raise ImportError("nuvec_b200/_native.so is missing: build it with `python -m nuvec_b200.build`")
         native.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SIGNATURES})
         _lib = handle
     return _lib

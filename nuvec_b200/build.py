@@ -1,5 +1,5 @@
-"""Builds libnuvec_cuda.so (the C-ABI CUDA backend) in-tree with nvcc for sm_100a, and _native.so (the operators' host
-path, CPython's C API) with g++.
+"""Builds libnuvec_cuda.so (the C-ABI CUDA backend) in-tree with nvcc for sm_100a, and the _native module (the operators'
+host path, CPython's C API) with g++.
 
 Usage: python -m nuvec_b200.build [--force] [--verbose] [--timeline]
 
@@ -8,6 +8,7 @@ Usage: python -m nuvec_b200.build [--force] [--verbose] [--timeline]
 """
 from __future__ import annotations
 
+import importlib
 import os
 import subprocess
 import sys
@@ -17,7 +18,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libnuvec_cuda.so"
-NATIVE = PKG / "_native.so"
+NATIVE = PKG / f"_native{sysconfig.get_config_var('EXT_SUFFIX')}"  # one per interpreter: its ABI is in the name
 TIMELINE_LIB = PKG / "libnuvec_cuda_timeline.so"
 SOURCES = ["runtime.cu", "quantize.cu", "qmv.cu", "qmm.cu", "qmm_bf16.cu", "qmm_f16.cu", "qmm_fp.cu", "qqmm.cu", "ops.cu", "moe.cu", "convert.cu", "attention.cu", "peer.cu", "comm_nccl.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -57,7 +58,7 @@ def build(force: bool = False, verbose: bool = False, timeline: bool = False) ->
         objs.append(str(obj))
     procs.append(("native.cpp", subprocess.Popen(
         ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}",
-         str(CSRC / "native.cpp"), "-o", str(NATIVE)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+         str(CSRC / "native.cpp"), "-o", str(build_dir / NATIVE.name)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, proc in procs:
         out, _ = proc.communicate()
@@ -68,8 +69,13 @@ def build(force: bool = False, verbose: bool = False, timeline: bool = False) ->
             sys.stderr.write(f"--- {src} ---\n{out}\n")
     if failed:
         raise RuntimeError("compilation failed")
-    link = [nvcc(), *ARCH, "-shared", "-o", str(lib), *objs, "-lcudart", "-ldl"]
+    link = [nvcc(), *ARCH, "-shared", "-o", str(build_dir / lib.name), *objs, "-lcudart", "-ldl"]
     subprocess.run(link, check=True)
+    for made in (lib, NATIVE):  # whole files change places: a process that has the old ones open keeps them
+        os.replace(build_dir / made.name, made)
+    importlib.invalidate_caches()
+    if "nuvec_b200._native" in sys.modules:
+        raise RuntimeError(f"{NATIVE.name} was rebuilt, but this process runs the one that it loaded before: start a new one")
     return lib
 
 

@@ -19,16 +19,6 @@ import numpy as np
 from . import _ffi
 from ._ffi import BF16, F16, F32, I32, U8, U32, native as _native
 
-
-class _NotBuilt:
-    """Stands for what csrc/native.cpp defines until it is built."""
-
-    def __init__(self, *args, **kwargs):
-        raise ImportError("nuvec_b200/_native.so is missing: build it with `python -m nuvec_b200.build`")
-
-
-_DeviceBase, _ArrayBase = (_native.DeviceBase, _native.ArrayBase) if _native else (_NotBuilt, _NotBuilt)
-
 __all__ = ["Device", "Array", "QuantMode", "Quant", "Quantized", "GatherQmm", "quantize", "dequantize",
            "quantized_matmul", "gather_qmm", "sorted_offsets", "moe_route", "weighted_sum", "expert_bias_add", "moe_sort", "take_rows", "swiglu", "swiglu_oai", "quantized_embedding", "rms_norm", "add_rms_norm", "quantized_attention", "fake_quant", "gather_qqmm", "qqmm", "qqmm_prepare_scales", "NuvecError", "InvalidArgument",
            "UnsupportedError", "OutOfMemory", "NoDevice", "BackendError", "CommError",
@@ -102,7 +92,7 @@ def promote_types(a: int, b: int) -> int:
 
 
 # ── device and arrays ──────────────────────────────────────────────────────────────────────
-class Device(_DeviceBase):
+class Device(_native.DeviceBase):
     """One GPU with its stream and pool (crates/nuvec-gpu/src/cuda/device.rs:77-227)."""
 
     _shared = {}
@@ -253,7 +243,7 @@ class Event:
             pass
 
 
-class Array(_ArrayBase):
+class Array(_native.ArrayBase):
     """A dense row-major device buffer with a shape and a dtype code (csrc/native.cpp holds the fields, ``reshape`` and
     ``[...]``: views that share another array's storage at a byte offset).
     """
@@ -375,8 +365,7 @@ class Quantized:
         return dequantize(self, dtype)
 
 
-if _native:
-    _native.register(Array, Quantized, tuple(QuantMode))
+_native.register(Array, Quantized, tuple(QuantMode))
 
 
 @dataclass(frozen=True)
