@@ -101,6 +101,9 @@ int32_t nvc_synchronize(nvc_device *dev);
 /* Adopts an existing cudaStream_t (for example the caller framework's current stream); NULL
  * returns to the handle's own stream.  The previous stream is synchronized first. */
 int32_t nvc_device_set_stream(nvc_device *dev, void *cuda_stream);
+/* The handle's stream.  Kernels of the handle read weights, caches and index lists before the kernel in
+ * front has finished when nothing unfinished writes them; on an adopted stream, and on the handle's
+ * own once it has been asked for here, that kernel may be the caller's, and nothing is read early. */
 void *nvc_device_stream(nvc_device *dev);
 /* Kernels this handle has launched so far (the reference counts dispatches the same way for
  * its tests, gpu.rs:27). */

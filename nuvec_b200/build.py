@@ -37,7 +37,7 @@ def stale(lib: Path = LIB) -> bool:
     if not lib.exists() or not NATIVE.exists():
         return True
     t = min(lib.stat().st_mtime, NATIVE.stat().st_mtime)
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + \
+    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cpp")) + \
         [PKG.parent / "include" / "nuvec_cuda.h", Path(__file__)]
     return any(d.stat().st_mtime > t for d in deps)
 

@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
         const int l = l0 + n / rep;
         return p.causal && n < rep * p.row_pack && l < p.L ? p.S - (p.L - 1 - l) : p.S;  // (columns that stand for nothing: any value)
     };
+    if (!p.early) pdl_wait();
     pdl_trigger();
 
     // This split's rows, addressed from its first by 32-bit byte offsets.
@@ -393,7 +394,6 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
     };
     const int first = warp * QM_STEP;
     constexpr int STRIDE = QM_WARPS * QM_STEP;
-    if (!p.early) pdl_wait();
 #pragma unroll
     for (int i = 0; i < STAGES - 1; i++) request(first + i * STRIDE, i);
     if (p.early) pdl_wait();  // (the caches may be read ahead of it, the queries not)
@@ -754,7 +754,8 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
     static_assert(BITS == 4 || BITS == 8, "codes that fill bytes");
     constexpr int W = D * BITS / 32, G = D / GS, KS = D / 16, NBD = D / 8, WP = W + 4;  // WP: padded row of the value tile
     constexpr int KS_PER_G = GS / 16, NBD_PER_G = GS / 8;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the combine kernel's blocks may become resident meanwhile
+    if (!p.early) pdl_wait();
+    pdl_trigger();  // the combine kernel's blocks may become resident meanwhile
     const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
     const int rep = p.Hq / p.Hkv, t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int g8 = lane >> 2, c = lane & 3;  // the fragments' group (a head, a key or a dim) and pair index
@@ -792,14 +793,11 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
 
     // The first tile's codes and scales start before the kernel in front has finished, unless it may be writing them.
     float4 nsb[G];
-    auto first_tile = [&]() {
-        if (s0 >= s1) return;
+    if (s0 < s1) {
         fetch_codes(s0, 0);
         fetch_scales(s0, nsb);
-    };
-    if (p.early) first_tile();
-    pdl_wait();
-    if (!p.early) first_tile();
+    }
+    if (p.early) pdl_wait();
     // the head's scaled queries as A fragments, and their sums per group (of the rounded values)
     uint32_t qa0[KS], qa2[KS];
     float qsum[G];
@@ -1029,18 +1027,8 @@ __global__ void __launch_bounds__(D) qattn_combine_kernel(QAttnParams p) {
 // The combine kernel, launched so that it may become resident while the split kernel runs (NUVEC_PDL=0: plain order).
 template <typename T, int D>
 static int32_t qattn_combine(nvc_device *dev, const QAttnParams &p) {
-    static const bool pdl = [] { const char *e = getenv("NUVEC_PDL"); return !(e && *e == '0'); }();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)p.Hq, (unsigned)p.B);
-    cfg.blockDim = dim3(D);
-    cfg.stream = dev->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    NVC_CUDA(cudaLaunchKernelEx(&cfg, qattn_combine_kernel<T, D>, p));
-    return check_launch(dev, "qattn_combine_kernel");
+    const Writes written(Trigger::LATE, {{p.out, (size_t)p.B * p.Hq * p.L * D * sizeof(T)}});
+    return launch_pdl(dev, "qattn_combine_kernel", written, qattn_combine_kernel<T, D>, dim3((unsigned)p.Hq, (unsigned)p.B), dim3(D), 0, p);
 }
 
 // The form of a call.  CUDA cores: float32 and 3-bit codes (NUVEC_QATTN_MMA=0: everything).  The ring form reads a row's scales
@@ -1076,8 +1064,11 @@ static int32_t qattn_launch_mma(nvc_device *dev, const QAttnParams &p, bool ring
             }
         }
         const dim3 grid((unsigned)p.splits, (unsigned)p.Hkv, (unsigned)(p.B * p.row_tiles));
-        if (ring) return launch_pdl(dev, "qattn_mma_kernel", qattn_mma_kernel<T, BITS, D, GS>, grid, dim3(QM_THREADS), ring_smem, p);
-        NVC_TRY(launch_pdl(dev, "qattn_tile_kernel", qattn_tile_kernel<T, BITS, D, GS>, grid, dim3(QA_THREADS), tile_smem, p));
+        const Trigger trigger = p.early ? Trigger::EARLY : Trigger::LATE;
+        if (ring)
+            return launch_pdl(dev, "qattn_mma_kernel", Writes(trigger, {{p.out, (size_t)p.B * p.Hq * p.L * D * sizeof(T)}}), qattn_mma_kernel<T, BITS, D, GS>, grid,
+                              dim3(QM_THREADS), ring_smem, p);
+        NVC_TRY(launch_pdl(dev, "qattn_tile_kernel", Writes(trigger, {}), qattn_tile_kernel<T, BITS, D, GS>, grid, dim3(QA_THREADS), tile_smem, p));
         return qattn_combine<T, D>(dev, p);
     }
     return set_error(NVC_ERR_UNSUPPORTED, "quantized_attention: no tensor-core kernel");

@@ -177,6 +177,7 @@ int32_t nvc_all_gather(nvc_comm *comm, const void *send, void *recv, size_t byte
     NVC_TRY(nvc::make_current(comm->dev));
     if (bytes_per_rank == 0) return NVC_OK;
     NVC_NCCL(settle(comm, g_api.AllGather(send, recv, bytes_per_rank, ncclUint8, comm->comm, comm->dev->stream)));
+    comm->dev->in_flight.unknown();
     return NVC_OK;
 }
 
@@ -197,6 +198,7 @@ int32_t nvc_recv(nvc_comm *comm, void *buf, size_t bytes, int32_t peer) {
     NVC_TRY(nvc::make_current(comm->dev));
     if (bytes == 0) return NVC_OK;
     NVC_NCCL(settle(comm, g_api.Recv(buf, bytes, ncclUint8, peer, comm->comm, comm->dev->stream)));
+    comm->dev->in_flight.unknown();
     return NVC_OK;
 }
 
@@ -220,6 +222,7 @@ int32_t nvc_all_reduce(nvc_comm *comm, int32_t op, int32_t dtype, void *buf, siz
     }
     if (count == 0) return NVC_OK;
     NVC_NCCL(settle(comm, g_api.AllReduce(buf, buf, count, t, rop, comm->comm, comm->dev->stream)));
+    comm->dev->in_flight.unknown();
     return NVC_OK;
 }
 

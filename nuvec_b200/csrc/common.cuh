@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/nuvec_cuda.h"
+#include "in_flight.h"
 
 namespace nvc {
 
@@ -86,10 +87,8 @@ struct nvc_device {
     size_t qmm_counters_len = 0;
     // Host-mapped word a kernel sets when one of its bounded waits gives up; read at synchronisation.
     int32_t *error_word = nullptr, *error_word_dev = nullptr;
-    // What triggering quantize launches may still be writing (see note_early_writer).
-    struct Range { const char *lo, *hi; };
-    Range early_writes[48];
-    int early_writes_n = 0;
+    nvc::InFlight in_flight;         // what unfinished kernels of the stream may be writing
+    bool stream_handed_out = false;  // nvc_device_stream was asked for: the stream may hold anybody's kernels
     // Asynchronous host-operand products: a pinned block (mapped into the device) and a device block
     // handed out front to back, and the results that wait in the pinned block for nvc_synchronize
     // to deliver them to the caller's memory.
@@ -126,7 +125,9 @@ int32_t make_current(nvc_device *dev);
 int32_t ensure_scratch(nvc_device *dev, size_t bytes, void **out);
 int32_t ensure_counters(nvc_device *dev, size_t count, uint32_t **out);
 int32_t check_quant(const char *op, const nvc_quant *q);
+// (a launch in plain stream order that says nothing of its writes: see in_flight.h)
 int32_t check_launch(nvc_device *dev, const char *kernel);
+int32_t check_launch(nvc_device *dev, const char *kernel, const Writes &writes, bool overlapping);
 // quantize.cu: bfloat16 x to nvfp4 / mxfp4 codes with the scales in the block-scaled MMA's layout (for qqmm.cu)
 int32_t quantize_fp4_laid(nvc_device *dev, const nvc_quant *q, const void *x, int64_t rows, int64_t cols, uint32_t *codes, uint8_t *laid,
                           int64_t kblocks, int pieces);
@@ -135,14 +136,16 @@ int32_t ensure_error_word(nvc_device *dev);  // the host-mapped word kernels rep
 
 // ── programmatic dependent launch ───────────────────────────────────────────────────────
 // A kernel launched with launch_pdl may start while its predecessor on the stream drains; it calls pdl_wait() before it
-// reads anything another kernel produces or writes anything.  pdl_trigger() lets the successor start: kernels that
-// produce activations call it at once, kernels whose results others read before their own wait (weights, index lists)
-// do not -- or their launches are noted, see early_read_ok.  NUVEC_PDL=0 restores plain stream order everywhere.
+// reads anything an unfinished kernel may write (early_read_ok) or writes anything.  pdl_trigger() lets the successor start.
+// Every launch says what it writes and whether it triggers before it waits (in_flight.h).  NUVEC_PDL=0 restores plain
+// stream order everywhere.
 bool pdl_enabled();
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
-int32_t launch_pdl_cluster(nvc_device *dev, const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A &&...args) {
+int32_t launch_pdl_cluster(nvc_device *dev, const char *name, const Writes &writes, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           unsigned cluster, A &&...args) {
+    const bool overlapping = pdl_enabled() && dev->in_flight.room(writes);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -150,7 +153,7 @@ int32_t launch_pdl_cluster(nvc_device *dev, const char *name, void (*kernel)(P..
     cfg.stream = dev->stream;
     cudaLaunchAttribute attr[2];
     unsigned n = 0;
-    if (pdl_enabled()) {
+    if (overlapping) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }
@@ -163,18 +166,14 @@ int32_t launch_pdl_cluster(nvc_device *dev, const char *name, void (*kernel)(P..
     cfg.attrs = attr;
     cfg.numAttrs = n;
     NVC_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
-    return check_launch(dev, name);
+    return check_launch(dev, name, writes, overlapping);
 }
 template <class... P, class... A>
-int32_t launch_pdl(nvc_device *dev, const char *name, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
-    return launch_pdl_cluster(dev, name, kernel, grid, block, smem, 1, static_cast<A &&>(args)...);
+int32_t launch_pdl(nvc_device *dev, const char *name, const Writes &writes, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+    return launch_pdl_cluster(dev, name, writes, kernel, grid, block, smem, 1, static_cast<A &&>(args)...);
 }
-// Products and attention read weights and caches before their pdl_wait().  That is safe unless a kernel still in flight
-// writes them.  The only triggering kernel that writes such arrays is quantize: note_early_writer keeps the ranges of
-// the launches since the last one that did not trigger (nothing starts before such a launch has finished) and says
-// whether this launch may trigger; early_read_ok says whether a range is clear of them (and the stream the handle's own:
-// on an adopted stream the kernel in front may be anybody's).
-bool note_early_writer(nvc_device *dev, const void *a, size_t an, const void *b, size_t bn, const void *c, size_t cn);
+// Whether the next kernel may read these bytes before its pdl_wait(): no unfinished kernel writes them, and the stream is the
+// handle's alone (on an adopted stream, or one handed out, the kernel in front may be anybody's).
 bool early_read_ok(const nvc_device *dev, const void *p, size_t n);
 
 inline size_t dtype_size(int32_t dtype) { return dtype == NVC_F32 ? 4 : 2; }

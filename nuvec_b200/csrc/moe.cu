@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(128) moe_route_warp_kernel(const T *__restrict
                                                              int64_t rows, int experts, int k, int normalize) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_trigger();
     pdl_wait();
     if (row >= rows) return;
     uint32_t key[PER];  // 0: taken, or no such expert
@@ -254,8 +255,8 @@ extern "C" int32_t nvc_moe_route(nvc_device *dev, int32_t dtype, const void *pro
     if (rows == 0) return NVC_OK;
     if (!probs || !out_indices || !out_scores) return set_error(NVC_ERR_INVALID_ARGUMENT, "moe_route: null operand");
     if (rows > 0x7FFFFFFFll) return set_error(NVC_ERR_UNSUPPORTED, "moe_route: %lld rows exceed the grid limit", (long long)rows);
-    // (no trigger: gathered products read the indices before their own wait)
     if (k <= ROUTE_WARP_MAX) {
+        const Writes written(Trigger::EARLY, {{out_indices, (size_t)(rows * k) * 4}, {out_scores, (size_t)(rows * k) * dtype_size(dtype)}});
         const dim3 grid((unsigned)((rows + 3) / 4));
 #define NVC_ROUTE(T)                                                                                                                     \
     {                                                                                                                                    \
@@ -263,7 +264,7 @@ extern "C" int32_t nvc_moe_route(nvc_device *dev, int32_t dtype, const void *pro
                       : experts <= 128 ? moe_route_warp_kernel<T, 4>                                                                     \
                       : experts <= 256 ? moe_route_warp_kernel<T, 8>                                                                     \
                                        : moe_route_warp_kernel<T, 32>;                                                                   \
-        return launch_pdl(dev, "moe_route_warp_kernel", kernel, grid, dim3(128), 0, (const T *)probs, out_indices, (T *)out_scores, rows, \
+        return launch_pdl(dev, "moe_route_warp_kernel", written, kernel, grid, dim3(128), 0, (const T *)probs, out_indices, (T *)out_scores, rows, \
                           (int)experts, (int)k, normalize);                                                                              \
     }
         switch (dtype) {
@@ -615,8 +616,9 @@ extern "C" int32_t nvc_weighted_sum(nvc_device *dev, int32_t dtype, const void *
     const unsigned threads = (unsigned)(cols >= 256 ? 256 : (cols + 31) / 32 * 32);
     const int64_t chunks = (cols + threads - 1) / threads;
     if (chunks > 65535) return set_error(NVC_ERR_UNSUPPORTED, "weighted_sum: %lld columns exceed the grid limit", (long long)d);
+    const Writes written(Trigger::EARLY, {{out, (size_t)(rows * d) * dtype_size(dtype)}});
 #define NVC_WSUM(T)                                                                                                                                 \
-    return launch_pdl(dev, "weighted_sum_kernel", wide ? weighted_sum_kernel<T, true> : weighted_sum_kernel<T, false>,                              \
+    return launch_pdl(dev, "weighted_sum_kernel", written, wide ? weighted_sum_kernel<T, true> : weighted_sum_kernel<T, false>,                              \
                       dim3((unsigned)rows, (unsigned)chunks), dim3(threads), 0, (const T *)x, (const T *)w, (T *)out, (int)k, d);
     switch (dtype) {
     case NVC_F32: NVC_WSUM(float)
@@ -637,8 +639,9 @@ extern "C" int32_t nvc_expert_bias_add(nvc_device *dev, int32_t dtype, void *y, 
     if (rows > 0x7FFFFFFFll) return set_error(NVC_ERR_UNSUPPORTED, "expert_bias_add: %lld rows exceed the grid limit", (long long)rows);
     const size_t item = dtype == NVC_F32 ? 4 : 2;
     const int wide = (n * item) % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)bias % 16 == 0;
+    const Writes written(Trigger::EARLY, {{y, (size_t)(rows * n) * item}});
 #define NVC_BIAS(T)                                                                                                                               \
-    return launch_pdl(dev, "expert_bias_add_kernel", expert_bias_add_kernel<T>, dim3((unsigned)rows), dim3(256), 0, (T *)y, (const T *)bias, indices, \
+    return launch_pdl(dev, "expert_bias_add_kernel", written, expert_bias_add_kernel<T>, dim3((unsigned)rows), dim3(256), 0, (T *)y, (const T *)bias, indices, \
                       n, (uint32_t)experts, wide);
     switch (dtype) {
     case NVC_F32: NVC_BIAS(float)
@@ -667,7 +670,9 @@ extern "C" int32_t nvc_moe_sort(nvc_device *dev, const uint32_t *indices, int64_
             configured[dev->ordinal] = true;
         }
     }
-    return launch_pdl(dev, "moe_sort_kernel", moe_sort_kernel, dim3(1), dim3(1024), smem, indices, pairs, (uint32_t)k, (uint32_t)experts, out_order,
+    const size_t list = (size_t)pairs * 4;
+    const Writes written(Trigger::LATE, {{out_order, list}, {out_restore, list}, {out_tokens, list}, {out_sorted, list}, {out_offsets, (size_t)experts * 4}});
+    return launch_pdl(dev, "moe_sort_kernel", written, moe_sort_kernel, dim3(1), dim3(1024), smem, indices, pairs, (uint32_t)k, (uint32_t)experts, out_order,
                       out_restore, out_tokens, out_sorted, out_offsets);
 }
 
@@ -679,8 +684,8 @@ extern "C" int32_t nvc_take_rows(nvc_device *dev, const void *src, int64_t src_r
     if (src_rows == 0) return set_error(NVC_ERR_INVALID_ARGUMENT, "take_rows: rows taken from an empty array");
     if (!src || !indices || !out) return set_error(NVC_ERR_INVALID_ARGUMENT, "take_rows: null operand");
     const int wide = row_bytes % 16 == 0 && (uintptr_t)src % 16 == 0 && (uintptr_t)out % 16 == 0;
-    // (no trigger: the rows may be anything, weights and index lists included)
-    return launch_pdl(dev, "take_rows_kernel", take_rows_kernel, dim3((unsigned)n), dim3(256), 0, (const uint8_t *)src, src_rows, row_bytes, indices,
+    const Writes written(Trigger::LATE, {{out, (size_t)(n * row_bytes)}});
+    return launch_pdl(dev, "take_rows_kernel", written, take_rows_kernel, dim3((unsigned)n), dim3(256), 0, (const uint8_t *)src, src_rows, row_bytes, indices,
                       (uint8_t *)out, wide);
 }
 
@@ -696,8 +701,9 @@ static int32_t launch_swiglu(nvc_device *dev, const char *op, int32_t dtype, con
     const int64_t per = wide ? 16 / (int64_t)dtype_size(dtype) : 1;
     const int64_t blocks = ((n + per - 1) / per + 255) / 256;
     if (blocks > 0x7FFFFFFFll) return set_error(NVC_ERR_UNSUPPORTED, "%s: %lld elements exceed the grid limit", op, (long long)n);
+    const Writes written(Trigger::EARLY, {{out, (size_t)n * dtype_size(dtype)}});
 #define NVC_SWIGLU(T, A, L)                                                                                                                        \
-    return launch_pdl(dev, "swiglu_kernel", wide ? swiglu_kernel<T, OAI, true> : swiglu_kernel<T, OAI, false>, dim3((unsigned)blocks), dim3(256), 0, \
+    return launch_pdl(dev, "swiglu_kernel", written, wide ? swiglu_kernel<T, OAI, true> : swiglu_kernel<T, OAI, false>, dim3((unsigned)blocks), dim3(256), 0, \
                       (const T *)gate, (const T *)up, (T *)out, n, A, L);
     // (the scalars are weak: rounded to the arrays' type, crates/nuvec-nn/src/lib.rs:504-507)
     switch (dtype) {
@@ -734,8 +740,10 @@ static int32_t launch_rms_norm(nvc_device *dev, const char *op, int32_t dtype, c
     const int nv = !wide ? 0 : pieces <= 1024 ? 1 : pieces <= 2048 ? 2 : 4;
     const int64_t want = nv ? (pieces + nv - 1) / nv : d;
     const unsigned threads = (unsigned)(want >= 1024 ? 1024 : (want + 31) / 32 * 32);
+    const size_t bytes = (size_t)(rows * d) * dtype_size(dtype);
+    const Writes written(Trigger::EARLY, {{y, bytes}, {sum_out, bytes}});
 #define NVC_RMS(T)                                                                                                                              \
-    return launch_pdl(dev, "rms_norm_kernel",                                                                                                   \
+    return launch_pdl(dev, "rms_norm_kernel", written,                                                                                                   \
                       nv == 0 ? rms_norm_kernel<T, 0> : nv == 1 ? rms_norm_kernel<T, 1> : nv == 2 ? rms_norm_kernel<T, 2> : rms_norm_kernel<T, 4>, \
                       dim3((unsigned)rows), dim3(threads), 0, (const T *)x, (const T *)residual, (const T *)weight, (T *)sum_out, (T *)y, d, eps, inv_count);
     switch (dtype) {

@@ -435,6 +435,7 @@ static int32_t host_batch(nvc_device *dev, const nvc_host_product *items, size_t
     if (!same_list) dev->batch_norecord = false;
     if (same && dev->batch_exec) {
         NVC_CUDA(cudaGraphLaunch(dev->batch_exec, dev->stream));
+        dev->in_flight.unknown();
         dev->launches += dev->batch_kernels;
         std::lock_guard<std::mutex> g(dev->host_mu);
         dev->pending.insert(dev->pending.end(), dev->batch_results.begin(), dev->batch_results.end());
@@ -454,11 +455,13 @@ static int32_t host_batch(nvc_device *dev, const nvc_host_product *items, size_t
         NVC_CUDA(cudaStreamBeginCapture(dev->stream, cudaStreamCaptureModeThreadLocal));
         dev->capturing = true;
         dev->captured = 0;
+        dev->in_flight.finished();  // (the recording's first kernel starts after everything in front of the replay)
     }
     // (leaves the recording, if one is open, before an error is returned)
     auto finish = [&](int32_t rc) -> int32_t {
         if (!record) return rc;
         dev->capturing = false;
+        dev->in_flight.unknown();
         cudaGraph_t graph = nullptr;
         cudaError_t err = cudaStreamEndCapture(dev->stream, &graph);
         if (rc == NVC_OK && err == cudaSuccess) {

@@ -167,6 +167,7 @@ extern "C" int32_t nvc_quantized_matmul_gather(nvc_device *dev, nvc_peer_group *
     if (overlaps(x, (size_t)(M * K) * 2, own + out_offset, foot))
         return set_error(NVC_ERR_INVALID_ARGUMENT, "quantized_matmul_gather: the activations overlap the product's own buffers");
     p.peer_mode = 1;
+    p.y = own + out_offset;  // (the kernel finds it through the regions' table; the launch notes what is written)
     p.peer_out_offset = out_offset;
     p.peer_ll_offset = out_offset + round256((size_t)group->host.size * (size_t)(M * N_local) * 2);
     return launch_qmv_affine(dev, q->bits, p, 1);

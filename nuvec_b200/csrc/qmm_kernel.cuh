@@ -134,7 +134,7 @@ struct QmmKernelParams {
     // A chunk's scales in shared memory: `chunk_bytes` of every row (s_pitch apart) in copies of s_vec bytes (16, 8, 4); rows
     // that are not 4-byte aligned are copied as the aligned words around them.  s_stages chunks fit the area.
     int32_t chunk_bytes, s_pitch, s_vec, s_stages;
-    int32_t early;                    // 1: nothing in flight writes the weights, they may be read before the wait for the previous kernel
+    int32_t early;                    // 1: nothing in flight writes the weights, they may be read before the wait for the previous kernel; 0: all wait first
 };
 
 // Instruction descriptor: D = f32, A = B = bf16 (or f16), both K-major, M = m, N = n.
@@ -588,6 +588,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     // A pair works as one: both blocks walk the same items.
     const int half = PAIR ? (int)pair_rank() : 0;
     const int block = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, blocks = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    if (!p.early) pdl_wait();
     pdl_trigger();
 
     if (tid == 0) {
@@ -705,7 +706,6 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
         QT_END(0, lane == 0)
     } else if (warp == 6) {
         // ── TMA producer, packed weights ────────────────────────────────────────────────────
-        if (!p.early) pdl_wait();
         const bool elected = elect_one();
         uint32_t s = 0, ph = 1;
         bool ok = true;
@@ -733,7 +733,6 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
         }
     } else if (warp >= QMM_SCALE_WARP) {
         // ── producers of scales and biases: a row per lane ──────────────────────────────────
-        if (!p.early) pdl_wait();
         const int r = (warp - QMM_SCALE_WARP) * 32 + lane;
         const uint32_t stage_bytes = (MODE == 0 ? 2 : 1) * 128 * p.s_pitch;
         int s = 0;
@@ -1227,7 +1226,8 @@ static int32_t launch_cfg(nvc_device *dev, const QmmParams &q, QmmKernelParams k
         k.partials = (float *)dev->qmm_partials;
         k.counters = dev->qmm_counters;
     }
-    return launch_pdl_cluster(dev, "qmm_kernel", kernel, dim3((unsigned)grid * (PAIR ? 2 : 1)), dim3(QMM_THREADS), S::SMEM, PAIR ? 2 : 1, mx, mw, k,
+    const Writes written(k.early ? Trigger::EARLY : Trigger::LATE, {{q.y, (size_t)q.rows * (size_t)q.N * 2}});
+    return launch_pdl_cluster(dev, "qmm_kernel", written, kernel, dim3((unsigned)grid * (PAIR ? 2 : 1)), dim3(QMM_THREADS), S::SMEM, PAIR ? 2 : 1, mx, mw, k,
                               (int)total_tiles, (int)n_tiles);
 }
 

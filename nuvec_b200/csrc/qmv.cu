@@ -673,6 +673,11 @@ __global__ void __launch_bounds__(WARPS * 32, QMV_BLOCKS_PER_SM * 8 / WARPS) qmv
     const int r = lane >> 2, t = lane & 3;
     const int64_t b = blockIdx.z;
     int64_t xb = b, wb = b;
+    // Programmatic dependent launch: the next kernel of the stream may be scheduled from now on, and this one reads its index
+    // lists and starts copying weights while the kernel before it is still finishing -- unless something unfinished may be
+    // writing them: then nothing is read before it has.
+    if (!p.early_weights) pdl_wait();
+    pdl_trigger();
     if (p.rhs) {
         // indices past the end select the last expert / activation batch, as the reference's `take`
         // clamps them (crates/nuvec-core/src/kernels.rs:120-129)
@@ -835,16 +840,6 @@ __global__ void __launch_bounds__(WARPS * 32, QMV_BLOCKS_PER_SM * 8 / WARPS) qmv
     // compile time.
     const uint32_t first_stage = (uint32_t)it_first % QMV_STAGES;
 
-    // Programmatic dependent launch: the next kernel of the stream may be scheduled from now on,
-    // and this one starts copying weights (which no product writes) while the kernel before it is
-    // still finishing; only then does it wait for that kernel's results.
-    if (p.early_weights) {
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    } else {
-        // the caller's stream may hold a kernel that writes these weights: nothing is read early
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
     if (lo < hi) {
         stage_scales(tile0, chunk0, 0);
         pf_rows(it_first);
@@ -852,8 +847,7 @@ __global__ void __launch_bounds__(WARPS * 32, QMV_BLOCKS_PER_SM * 8 / WARPS) qmv
 #pragma unroll
     for (int st = 0; st < QMV_STAGES; st++) prefetch(ring_s + ((first_stage + st) % QMV_STAGES) * STAGE_BYTES);
     QMV_TIMELINE_MARK(1)
-    if (p.early_weights)
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // activations, scratch and output belong to this kernel from here
+    if (p.early_weights) pdl_wait();  // activations, scratch and output belong to this kernel from here
     QMV_TIMELINE_MARK(2)
     // ── stage the activations once per block (the first weight copies are already in flight) ──
     {
@@ -1352,8 +1346,13 @@ static int32_t launch_qmv_cfg(nvc_device *dev, QmvParams &p, dim3 grid, size_t s
     const int64_t matrices = p.rhs ? (int64_t)p.experts : (int64_t)grid.z;
     const size_t w_bytes = (size_t)((matrices - 1) * p.w_batch_stride + p.N * (int64_t)p.row_words) * 4;
     const size_t s_bytes = (size_t)((matrices - 1) * p.s_batch_stride + p.N * (int64_t)p.row_groups) * (p.biases ? 2 : 1);
-    p.early_weights = early_read_ok(dev, p.w, w_bytes) && early_read_ok(dev, p.scales, s_bytes) && (!p.biases || early_read_ok(dev, p.biases, s_bytes));
-    return launch_pdl(dev, "qmv_affine_kernel", kernel, grid, dim3(WARPS * 32), smem, p);
+    const size_t list = (size_t)grid.z * 4, globals = p.expert_global ? (size_t)matrices * 4 : 4;
+    p.early_weights = early_read_ok(dev, p.w, w_bytes) && early_read_ok(dev, p.scales, s_bytes) && (!p.biases || early_read_ok(dev, p.biases, s_bytes)) &&
+                      (!p.rhs || early_read_ok(dev, p.rhs, list)) && (!p.lhs || early_read_ok(dev, p.lhs, list)) &&
+                      (!p.global || early_read_ok(dev, p.global, globals));
+    const Writes written(p.early_weights ? Trigger::EARLY : Trigger::LATE,
+                         {{p.y, (size_t)grid.z * (size_t)(p.M * p.N) * 2 * (size_t)(p.peer_mode == 1 ? p.peer_size : 1)}});
+    return launch_pdl(dev, "qmv_affine_kernel", written, kernel, grid, dim3(WARPS * 32), smem, p);
 }
 
 int32_t launch_qmv_affine(nvc_device *dev, int32_t bits, QmvParams p, int64_t batch, const QmvScratch *fixed) {

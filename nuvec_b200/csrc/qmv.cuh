@@ -53,8 +53,8 @@ struct QmvParams {
     // Gathers: number of weight batches and activation batches the index lists may address; an index
     // past the end selects the last one (the reference's `take` clamps).  0 - 1 = no limit.
     uint32_t experts, x_batches;
-    // 1: weights, scales and biases may be read before the previous kernel of the stream has
-    // finished (they are constants of the stream's work); 0: nothing is read before it has.
+    // 1: weights, scales, biases, index lists and global scales may be read before the previous kernel of
+    // the stream has finished (nothing unfinished writes them); 0: nothing is read before it has.
     int32_t early_weights;
     const float *global;       // nvfp4 global scale(s) or nullptr
     int32_t expert_global;     // one value per expert (indexed like the weights' batch)

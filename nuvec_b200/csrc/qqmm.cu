@@ -351,19 +351,8 @@ static int32_t qq_launch(nvc_device *dev, const CUtensorMap &mw, const CUtensorM
     // Programmatic stream serialization: the blocks may start (barriers, tensor memory, descriptors) while the kernel
     // before this one, the activations' quantization, drains; the producer thread synchronises with it on the device
     // (griddepcontrol.wait) before its first load.  NUVEC_PDL=0 restores plain stream order.
-    static const bool pdl = [] { const char *e = getenv("NUVEC_PDL"); return !(e && *e == '0'); }();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(QQ_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = dev->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    NVC_CUDA(cudaLaunchKernelEx(&cfg, kernel, mw, mx, p));
-    return check_launch(dev, "qqmm_kernel");
+    const Writes written(Trigger::LATE, {{p.y, (size_t)tokens * (size_t)N * 2}});
+    return launch_pdl(dev, "qqmm_kernel", written, kernel, grid, dim3(QQ_THREADS), smem, mw, mx, p);
 }
 
 }  // namespace nvc

@@ -142,9 +142,10 @@ template <typename T, bool FUSED>
 static int32_t launch_dequantize_affine(nvc_device *dev, int bits, const uint8_t *codes, const void *scales,
                                         const void *biases, void *out, size_t packs, int gs_shift, RowPick pick) {
     const int wide = (uintptr_t)out % 16 == 0;
+    const Writes written(Trigger::LATE, {{out, packs * 8 * sizeof(T)}});
 #define NVC_CASE(B)                                                                                                                     \
     case B:                                                                                                                             \
-        return launch_pdl(dev, "dequantize_affine_kernel",                                                                              \
+        return launch_pdl(dev, "dequantize_affine_kernel", written,                                                                              \
                           pick.ids ? dequantize_affine_kernel<T, B, FUSED, true> : dequantize_affine_kernel<T, B, FUSED, false>,        \
                           pack_grid(packs, pick), dim3(256), 0, codes, (const T *)scales, (const T *)biases, (T *)out, packs, gs_shift, pick, wide);
     switch (bits) {
@@ -184,9 +185,9 @@ __device__ __forceinline__ float near_half_code(float x, float scale, float r, f
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256)
 quantize_affine_kernel(const T *__restrict__ w, uint8_t *__restrict__ codes, T *__restrict__ scales,
-                       T *__restrict__ biases, size_t packs, int lanes, int wide, int trigger) {
+                       T *__restrict__ biases, size_t packs, int lanes, int wide) {
     constexpr int V = 16, QUADS = V * (int)sizeof(T) / 16;
-    if (trigger) pdl_trigger();
+    pdl_trigger();
     const size_t at = (size_t)blockIdx.x * 256 + threadIdx.x;
     const bool have = at < packs;
     const size_t i = have ? at : packs - 1;  // (whole groups past the end: their lanes repeat the last pack and store nothing)
@@ -344,9 +345,9 @@ struct ScalePieces {
 template <typename T, int BITS, int GS, bool LAID = false>
 __global__ void __launch_bounds__(256)
 quantize_fp_kernel(const T *__restrict__ w, uint8_t *__restrict__ codes, uint8_t *__restrict__ scales,
-                   const float *__restrict__ global, size_t packs, int trigger, ScalePieces sp = ScalePieces{}) {
+                   const float *__restrict__ global, size_t packs, ScalePieces sp = ScalePieces{}) {
     constexpr int V = 16, QUADS = V * (int)sizeof(T) / 16, LANES = GS / V;
-    if (LAID || trigger) pdl_trigger();  // (LAID: the product kernel may set itself up meanwhile)
+    pdl_trigger();  // (LAID: the product kernel may set itself up meanwhile)
     size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;  // this thread's pack of V values
     bool have = i < packs;
     size_t laid_at = 0;
@@ -437,14 +438,14 @@ template <typename T>
 static int32_t quantize_typed(nvc_device *dev, const nvc_quant *q, const void *w, size_t count,
                               const float *global, uint32_t *codes, void *scales, void *biases) {
     const size_t groups = count / (size_t)q->group_size, scale_bytes = groups * (q->mode == NVC_AFFINE ? sizeof(T) : 1);
-    const int trigger = note_early_writer(dev, codes, count * (size_t)q->bits / 8, scales, scale_bytes, biases, scale_bytes);
+    const Writes written(Trigger::EARLY, {{codes, count * (size_t)q->bits / 8}, {scales, scale_bytes}, {biases, scale_bytes}});
     if (q->mode == NVC_AFFINE) {
         const size_t packs = count / 16;
         const int lanes = q->group_size / 16, wide = (uintptr_t)w % 16 == 0;
 #define NVC_CASE(B)                                                                                                                          \
     case B:                                                                                                                                  \
-        return launch_pdl(dev, "quantize_affine_kernel", quantize_affine_kernel<T, B>, dim3((unsigned)((packs + 255) / 256)), dim3(256), 0, \
-                          (const T *)w, (uint8_t *)codes, (T *)scales, (T *)biases, packs, lanes, wide, trigger);
+        return launch_pdl(dev, "quantize_affine_kernel", written, quantize_affine_kernel<T, B>, dim3((unsigned)((packs + 255) / 256)), dim3(256), 0, \
+                          (const T *)w, (uint8_t *)codes, (T *)scales, (T *)biases, packs, lanes, wide);
         switch (q->bits) {
             NVC_CASE(1) NVC_CASE(2) NVC_CASE(3) NVC_CASE(4) NVC_CASE(5) NVC_CASE(6) NVC_CASE(8)
         default: return set_error(NVC_ERR_INVALID_ARGUMENT, "quantize: %d bits", q->bits);
@@ -452,10 +453,10 @@ static int32_t quantize_typed(nvc_device *dev, const nvc_quant *q, const void *w
 #undef NVC_CASE
     }
     const size_t packs = count / 16;
-    return launch_pdl(dev, "quantize_fp_kernel",
+    return launch_pdl(dev, "quantize_fp_kernel", written,
                       q->bits == 8 ? quantize_fp_kernel<T, 8, 32> : q->group_size == 16 ? quantize_fp_kernel<T, 4, 16> : quantize_fp_kernel<T, 4, 32>,
                       dim3((unsigned)((packs + 255) / 256)), dim3(256), 0, (const T *)w, (uint8_t *)codes, (uint8_t *)scales, global, packs,
-                      trigger, ScalePieces{});
+                      ScalePieces{});
 }
 
 template <typename T>
@@ -472,7 +473,7 @@ static int32_t dequantize_typed(nvc_device *dev, const nvc_quant *q, const uint3
     const int wide = (uintptr_t)out % 16 == 0;
     auto kernel = q->bits == 4 ? (pick.ids ? dequantize_fp_kernel<T, 4, true> : dequantize_fp_kernel<T, 4, false>)
                                : (pick.ids ? dequantize_fp_kernel<T, 8, true> : dequantize_fp_kernel<T, 8, false>);
-    return launch_pdl(dev, "dequantize_fp_kernel", kernel, pack_grid(packs, pick), dim3(256), 0, bytes, (const uint8_t *)scales, global, (T *)out,
+    return launch_pdl(dev, "dequantize_fp_kernel", Writes(Trigger::LATE, {{out, packs * 8 * sizeof(T)}}), kernel, pack_grid(packs, pick), dim3(256), 0, bytes, (const uint8_t *)scales, global, (T *)out,
                       packs, gs_shift, pick, wide);
 }
 
@@ -560,10 +561,11 @@ int32_t nvc::quantize_fp4_laid(nvc_device *dev, const nvc_quant *q, const void *
     const int64_t padded_rows = (rows + 127) / 128 * 128, padded_groups = kblocks * pieces * 4;
     const size_t threads = (size_t)padded_rows * (size_t)padded_groups * (size_t)(q->group_size / 16);
     ScalePieces sp{laid, rows, cols / q->group_size, kblocks, pieces};
-    return launch_pdl(dev, "quantize_fp_kernel",
+    const Writes written(Trigger::EARLY, {{codes, (size_t)(rows * cols / 2)}, {laid, (size_t)(padded_rows / 128 * kblocks) * pieces * 512}});
+    return launch_pdl(dev, "quantize_fp_kernel", written,
                       q->group_size == 16 ? quantize_fp_kernel<__nv_bfloat16, 4, 16, true> : quantize_fp_kernel<__nv_bfloat16, 4, 32, true>,
                       dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, (const __nv_bfloat16 *)x, (uint8_t *)codes, nullptr, nullptr, (size_t)0,
-                      1, sp);
+                      sp);
 }
 
 // FastOp::QuantizeDequantize (crates/nuvec-core/src/products.rs:306-315, MLX's fp_quantize_dequantize): x through

@@ -33,7 +33,7 @@ int32_t make_current(nvc_device *dev) {
     return NVC_OK;
 }
 
-int32_t check_launch(nvc_device *dev, const char *kernel) {
+static int32_t count_launch(nvc_device *dev, const char *kernel) {
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess)
         return set_error(NVC_ERR_DRIVER, "launch of %s failed: %s", kernel, cudaGetErrorString(err));
@@ -42,32 +42,25 @@ int32_t check_launch(nvc_device *dev, const char *kernel) {
     return NVC_OK;
 }
 
+int32_t check_launch(nvc_device *dev, const char *kernel) {
+    NVC_TRY(count_launch(dev, kernel));
+    dev->in_flight.unknown();
+    return NVC_OK;
+}
+
+int32_t check_launch(nvc_device *dev, const char *kernel, const Writes &writes, bool overlapping) {
+    NVC_TRY(count_launch(dev, kernel));
+    dev->in_flight.note(writes, overlapping);
+    return NVC_OK;
+}
+
 bool pdl_enabled() {
     static const bool on = [] { const char *e = getenv("NUVEC_PDL"); return !(e && *e == '0'); }();
     return on;
 }
 
-bool note_early_writer(nvc_device *dev, const void *a, size_t an, const void *b, size_t bn, const void *c, size_t cn) {
-    constexpr int room = (int)(sizeof dev->early_writes / sizeof dev->early_writes[0]);
-    if (dev->early_writes_n + 3 > room) {  // no room to remember it: this launch does not trigger, and so ends all of them
-        dev->early_writes_n = 0;
-        return false;
-    }
-    auto add = [&](const void *p, size_t n) {
-        if (p && n) dev->early_writes[dev->early_writes_n++] = {(const char *)p, (const char *)p + n};
-    };
-    add(a, an);
-    add(b, bn);
-    add(c, cn);
-    return true;
-}
-
 bool early_read_ok(const nvc_device *dev, const void *p, size_t n) {
-    if (dev->stream != dev->own_stream) return false;
-    const char *lo = (const char *)p, *hi = lo + n;
-    for (int i = 0; i < dev->early_writes_n; i++)
-        if (lo < dev->early_writes[i].hi && dev->early_writes[i].lo < hi) return false;
-    return true;
+    return dev->stream == dev->own_stream && !dev->stream_handed_out && dev->in_flight.clear_of(p, n);
 }
 
 int32_t deliver_pending(nvc_device *dev) {
@@ -325,7 +318,7 @@ int32_t nvc_device_info(nvc_device *dev, nvc_info *out) {
 int32_t nvc_synchronize(nvc_device *dev) {
     NVC_TRY(make_current(dev));
     NVC_CUDA(cudaStreamSynchronize(dev->stream));
-    dev->early_writes_n = 0;  // nothing is in flight
+    dev->in_flight.finished();
     deliver_pending(dev);
     if (dev->error_word && *dev->error_word != 0) {
         *dev->error_word = 0;
@@ -343,10 +336,15 @@ int32_t nvc_device_set_stream(nvc_device *dev, void *cuda_stream) {
     NVC_TRY(make_current(dev));
     NVC_CUDA(cudaStreamSynchronize(dev->stream));
     dev->stream = cuda_stream ? (cudaStream_t)cuda_stream : dev->own_stream;
+    dev->in_flight.finished();
     return NVC_OK;
 }
 
-void *nvc_device_stream(nvc_device *dev) { return dev ? (void *)dev->stream : nullptr; }
+void *nvc_device_stream(nvc_device *dev) {
+    if (!dev) return nullptr;
+    if (dev->stream == dev->own_stream) dev->stream_handed_out = true;
+    return (void *)dev->stream;
+}
 uint64_t nvc_launch_count(nvc_device *dev) { return dev ? dev->launches : 0; }
 
 int32_t nvc_alloc(nvc_device *dev, size_t bytes, void **out) {
@@ -478,6 +476,7 @@ int32_t nvc_graph_begin(nvc_device *dev) {
     NVC_CUDA(cudaStreamBeginCapture(dev->stream, cudaStreamCaptureModeThreadLocal));
     dev->capturing = true;
     dev->captured = 0;
+    dev->in_flight.finished();  // (a recording's first kernel starts after everything in front of the replay)
     return NVC_OK;
 }
 
@@ -487,6 +486,7 @@ int32_t nvc_graph_end(nvc_device *dev, nvc_graph **out) {
     NVC_TRY(make_current(dev));
     if (!dev->capturing) return set_error(NVC_ERR_INVALID_ARGUMENT, "nvc_graph_end: not recording");
     dev->capturing = false;
+    dev->in_flight.unknown();  // (of the work that was enqueued before the recording began)
     cudaGraph_t graph = nullptr;
     NVC_CUDA(cudaStreamEndCapture(dev->stream, &graph));
     nvc_graph *g = new nvc_graph();
@@ -509,6 +509,7 @@ int32_t nvc_graph_launch(nvc_device *dev, nvc_graph *graph) {
     NVC_TRY(make_current(dev));
     NVC_CUDA(cudaGraphLaunch(graph->exec, dev->stream));
     dev->launches += graph->kernels;
+    dev->in_flight.unknown();
     return NVC_OK;
 }
 

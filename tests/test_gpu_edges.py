@@ -176,3 +176,64 @@ def test_few_rows_staged_across_rows(be, fmt):
         flat = be.up(np.concatenate([np.zeros(3, x.dtype), x.reshape(-1)]), NVC[dt])  # the same rows, 6 bytes into an allocation
         got = host(nv.quantized_matmul(flat[3:].reshape(M, K), be.quantized(c, s, b, NVC[dt], mode, gs, bits)))
         assert same(got, dense[:, ks].T, dt), (N, K)
+
+
+# ── reads ahead of the wait for the kernel in front ─────────────────────────────────────────
+@pytest.mark.parametrize("path", ["few rows", "many rows", "gather", "grouped", "attention", "attention rows"])
+def test_operands_that_the_kernels_in_front_have_just_written(be, path):
+    """Weights, scales, lists and caches come from launches directly in front or one kernel further, into blocks that held
+    other values a moment ago: the results are those with an idle stream before every launch, eagerly and recorded."""
+    rng = np.random.default_rng(3)
+    N, K, E = 96, 512, 8
+    quant = nv.Quant.affine(64, 4)
+    table = nv.quantize(be.up(oracle.from_f32(rng.standard_normal((8 * N, K)).astype(np.float32), oracle.BF16), nv.BF16), quant)
+    picks = [be.up(rng.permutation(8 * N)[:4 * N].astype(np.uint32), nv.U32) for _ in range(6)]
+    x = be.up(oracle.from_f32(rng.standard_normal((40, K)).astype(np.float32), oracle.BF16), nv.BF16)
+    rows = 4 if path == "attention rows" else 1
+
+    def step(pick, pause, between):
+        parts = []
+        for a in (table.scales, table.biases, table.weight):
+            parts.append(nv.take_rows(a, pick))
+            pause()
+        q = nv.Quantized(parts[2], parts[0], parts[1], quant)
+        h = x[:40 if path in ("many rows", "grouped") else 4]
+        if between:  # a kernel that lets the product start before it has waited itself
+            h = nv.rms_norm(h)
+            pause()
+        if path in ("few rows", "many rows"):
+            y = nv.quantized_matmul(h, q)
+        elif path in ("gather", "grouped"):
+            experts = nv.Quantized(*(a.reshape(E, -1, a.shape[-1]) for a in (q.weight, q.scales, q.biases)), quant)
+            probs = nv.quantized_matmul(h, nv.Quantized(q.weight[:E], q.scales[:E], q.biases[:E], quant))
+            pause()
+            idx, _ = nv.moe_route(probs, 2)
+            pause()
+            if path == "gather":
+                y = nv.gather_qmm(h.reshape(4, 1, K), experts, lhs, idx)
+            else:
+                order, _, tokens, ids, offs = nv.moe_sort(idx, E)
+                pause()
+                mine = nv.take_rows(h, tokens)
+                pause()
+                y = nv.gather_qmm(mine.reshape(80, 1, K), experts, None, ids, nv.GatherQmm(sorted_indices=True), offs)
+        else:
+            heads = 2 if path == "attention" else 1  # 1536 or 3072 keys of 64
+            k = nv.Quantized(*(a.reshape(1, heads, -1, a.shape[-1] // 8) for a in (q.weight, q.scales, q.biases)), quant)
+            y = nv.quantized_attention(h[:rows].reshape(1, 8, rows, 64), k, k, 0.125)
+        pause()
+        return y, parts
+
+    lhs = be.up(np.repeat(np.arange(4, dtype=np.uint32), 2).reshape(4, 2), nv.U32)
+    for between in (False, True):
+        want = [host(step(p, be.dev.synchronize, between)[0]) for p in picks]
+        for _ in range(3):
+            kept = [step(p, lambda: None, between) for p in picks]
+            for (g, _), w in zip(kept, want):
+                assert np.array_equal(host(g), w), (path, between, "eager")
+        kept = []  # (the blocks go back to the pool, which cannot grow while recording)
+        graph = be.dev.record(lambda: kept.extend(step(p, lambda: None, between) for p in picks))
+        for _ in range(3):
+            graph.launch()
+            for (g, _), w in zip(kept, want):
+                assert np.array_equal(host(g), w), (path, between, "recorded")
