@@ -26,6 +26,7 @@
 
 #include <cstdlib>
 #include <initializer_list>
+#include <type_traits>
 
 namespace nvc {
 
@@ -240,7 +241,8 @@ __global__ void __launch_bounds__(QA_THREADS, 5) qattn_split_kernel(QAttnParams 
 //   values   O[d, n] += sum over keys of (1024 + code[key, d]) * (p[key, n] * s_g(d)[key])
 //            out[d, n] = O[d, n] + sum over keys of (p * b_g(d)[key] - 1024 * p * s_g(d)[key])
 // A code enters as the exact float16 integer 1024 + code (one byte permutation per pair at 8 bits, a shift and a LOP3 at 4),
-// and the offset leaves with sums the kernel keeps anyway.  q * scale and p * s are rounded to float16.
+// and the offset leaves with sums the kernel keeps anyway.  q * scale and p * s are rounded to float16, the latter where float16
+// has all its bits (QA_TOP).
 //
 // Every warp works alone on steps of 16 keys: no barrier before the end.  The order of the dims in a dot
 // product and of the dims among the output rows is free, so every lane's share of a row is contiguous bytes, all of which
@@ -273,7 +275,17 @@ __device__ __forceinline__ float qa_exp2(float x) {  // 2 to the x, relative err
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-constexpr float QA_SLACK = 3.0f;
+// p * s has to pass through float16.  The exponents' reference point is therefore placed by the value scales too: with
+// 2^k the power of two at or above the largest scale met so far, the largest p * s lies between 2^11 and 2^15, 25 binary
+// orders above float16's subnormals.  (With p <= 1 as the softmax has it, values of magnitude 10^-3 lose most of their codes:
+// relative error 0.86 at 16K keys, 8 bits.)  It is a score plus a whole number: the key that set it has a power of two for its p,
+// and so an exact p * s (whole reference points: peaked scores 8e-4 off instead of 5e-4).
+constexpr float QA_SLACK = 3.0f, QA_TOP = 15.0f;  // room above the largest score when the reference moves; log2 of the largest p * s
+constexpr int QA_K_MIN = -26, QA_K_MAX = 55;      // scales outside are taken as these: sums of 2^(QA_TOP - k) * p stay in float32's range
+__device__ __forceinline__ int qa_log2_ceil(float s) {  // of s >= 0, in [QA_K_MIN, QA_K_MAX]
+    const uint32_t u = __float_as_uint(s);
+    return min(max((int)(u >> 23) - 127 + ((u & 0x7FFFFFu) != 0u ? 1 : 0), QA_K_MIN), QA_K_MAX);
+}
 __device__ __forceinline__ uint32_t qa_nibbles(uint32_t v) { return (v & 0x000F000Fu) | 0x64006400u; }
 template <int WORDS> __device__ __forceinline__ void qa_load(const void *src, uint32_t *dst) {
     if constexpr (WORDS == 4) {
@@ -298,7 +310,26 @@ template <typename T, int G> struct QaScales {
         const uint16_t h = (uint16_t)(raw[g >> 1] >> (16 * (g & 1)));
         return DT<T>::load(reinterpret_cast<const T *>(&h), 0);
     }
+    // the magnitudes here and in `other`, as the larger of each pair of half words: their bits are in order
+    __device__ __forceinline__ uint32_t largest(const QaScales &other) const {
+        uint32_t u = __vmaxu2(raw[0] & 0x7FFF7FFFu, other.raw[0] & 0x7FFF7FFFu);
+        if (G == 4) u = __vmaxu2(u, __vmaxu2(raw[G / 4] & 0x7FFF7FFFu, other.raw[G / 4] & 0x7FFF7FFFu));
+        return u;
+    }
 };
+// k of the larger of two magnitudes (zero, infinities and NaN: no scale to go by), and 2^k as both half words
+template <typename T> __device__ __forceinline__ int qa_scale_k(uint32_t pair) {
+    constexpr uint32_t INF = std::is_same<T, __half>::value ? 0x7C00u : 0x7F80u;
+    const uint32_t a = pair >> 16, b = pair & 0xFFFFu;
+    const uint16_t h = (uint16_t)max(a < INF ? a : 0u, b < INF ? b : 0u);
+    return qa_log2_ceil(DT<T>::load(reinterpret_cast<const T *>(&h), 0));
+}
+template <typename T> __device__ __forceinline__ uint32_t qa_scale_pair(int k) {
+    T h[2];
+    DT<T>::store(h, 0, __uint_as_float((uint32_t)(k + 127) << 23));
+    h[1] = h[0];
+    return *reinterpret_cast<const uint32_t *>(h);
+}
 
 constexpr int QM_WARPS = 8, QM_THREADS = QM_WARPS * 32, QM_STEP = 16;  // keys per step of a warp
 constexpr int QM_BLOCKS_PER_SM = 2;
@@ -439,8 +470,10 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
     const int limit[2] = {limit_of(2 * c) - s0, limit_of(2 * c + 1) - s0};
     const int all_of = min(s1, p.causal ? p.S - (p.L - 1 - l0) : p.S) - s0;  // every column attends to the keys before this one
 
-    // m: the reference point of the exponents, at least the largest score so far minus QA_SLACK
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};  // of columns 2c, 2c + 1 (l: this lane's keys only)
+    // top: no score so far is above it; ref = top - (QA_TOP - k): the reference point of the exponents
+    float top[2] = {-INFINITY, -INFINITY}, ref[2] = {0.0f, 0.0f}, l[2] = {0.0f, 0.0f};  // of columns 2c, 2c + 1 (l: this lane's keys only)
+    int k = QA_K_MIN;
+    uint32_t largest = 0u;  // 2^k in the scales' type, twice (0 to begin with)
     float o[G][MT][4], side[G][2];
 #pragma unroll
     for (int gr = 0; gr < G; gr++) {
@@ -507,20 +540,33 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
             for (int i = 0; i < 4; i++)
                 if (key0 + g + 8 * (i >> 1) >= min(limit[i & 1], last + 1)) sc[i] = -INFINITY;
         }
-        // The exponents' reference point moves only when a score exceeds it by more than QA_SLACK: rescaling the outputs at every
-        // new maximum, and finding it across the lanes, took a third of the step.  It is subtracted with the slack, so that
-        // no probability is above one.
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            vsc[r].load(at + 2 * R::CODES + 2 * R::SPIECE + off[2] + (g + 8 * r) * 2 * G);
+            vbi[r].load(at + 2 * R::CODES + 3 * R::SPIECE + off[3] + (g + 8 * r) * 2 * G);
+            // one group: the last row's word also holds a value that is not the cache's; a probability of zero times that may be NaN
+            if (G == 1 && key0 + g + 8 * r > last) vsc[r].raw[0] = vbi[r].raw[0] = 0u;
+        }
+        // The exponents' reference point moves only when a score passes `top`, which has QA_SLACK of room when it is set, or a
+        // scale the largest so far: rescaling the outputs at every new maximum, and finding it across the lanes, took a third of
+        // the step.
         const float mx[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
-        if (__any_sync(0xFFFFFFFFu, mx[0] > m[0] + QA_SLACK || mx[1] > m[1] + QA_SLACK)) {
+        const uint32_t vs = vsc[0].largest(vsc[1]);
+        if (__any_sync(0xFFFFFFFFu, mx[0] > top[0] || mx[1] > top[1] || __vmaxu2(vs, largest) != largest)) {
             float corr[2];
+            k = max(k, __reduce_max_sync(0xFFFFFFFFu, qa_scale_k<T>(vs)));
+            largest = qa_scale_pair<T>(k);
+            const float head = QA_TOP - (float)k;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 float n = mx[i];
 #pragma unroll
                 for (int s = 4; s < 32; s <<= 1) n = fmaxf(n, __shfl_xor_sync(0xFFFFFFFFu, n, s));
-                n = fmaxf(m[i], n);
-                corr[i] = m[i] == -INFINITY ? 0.0f : qa_exp2(m[i] - n);
-                m[i] = n;
+                n = n > top[i] ? n + QA_SLACK : top[i];
+                const float to = n == -INFINITY ? 0.0f : n - head;
+                corr[i] = top[i] == -INFINITY ? 0.0f : qa_exp2(ref[i] - to);
+                top[i] = n;
+                ref[i] = to;
                 l[i] *= corr[i];
             }
 #pragma unroll
@@ -534,7 +580,6 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
                 }
             }
         }
-        const float ref[2] = {m[0] == -INFINITY ? 0.0f : m[0] + QA_SLACK, m[1] == -INFINITY ? 0.0f : m[1] + QA_SLACK};
         float pr[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -542,13 +587,6 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
             l[i & 1] += pr[i];
         }
         // ── values ──
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            vsc[r].load(at + 2 * R::CODES + 2 * R::SPIECE + off[2] + (g + 8 * r) * 2 * G);
-            vbi[r].load(at + 2 * R::CODES + 3 * R::SPIECE + off[3] + (g + 8 * r) * 2 * G);
-            // one group: the last row's word also holds a value that is not the cache's; a probability of zero times that may be NaN
-            if (G == 1 && key0 + g + 8 * r > last) vsc[r].raw[0] = vbi[r].raw[0] = 0u;
-        }
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -618,7 +656,7 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
     if (g == 0) {
 #pragma unroll
         for (int n = 0; n < 2; n++) {
-            wm[warp][2 * c + n] = m[n] == -INFINITY ? -INFINITY : m[n] + QA_SLACK;
+            wm[warp][2 * c + n] = top[n] == -INFINITY ? -INFINITY : ref[n];
             wl[warp][2 * c + n] = l[n];
         }
     }
@@ -739,7 +777,8 @@ __global__ void __launch_bounds__(QM_THREADS, QM_BLOCKS_PER_SM) qattn_mma_kernel
 // value products, so the probabilities never leave registers; the four warps' outputs are added at the end.  A tile's codes
 // travel into shared memory with cp.async a tile ahead (two sets of buffers), its scales and biases through registers; the
 // splits are merged by qattn_combine.  See qattn_form for when it runs.
-constexpr int QT_BLOCKS = 3;
+constexpr int QT_BLOCKS = 3, QT_PLAIN = 7;
+__device__ __forceinline__ float qa_inverse(float x) { return __uint_as_float((254u << 23) - __float_as_uint(x)); }  // of a power of two
 __device__ __forceinline__ void qa_cp16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -821,16 +860,29 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
     }
 
     float m = -INFINITY, l = 0.0f;  // of head g8
-    float oc[NBD][4], side[G];      // outputs [head g8][dims 8 nbd + 2 c, + 1] (rows 8-15 idle); bias / offset terms per group
+    float oc[NBD][4], side[G];      // outputs times `lift` [head g8][dims 8 nbd + 2 c, + 1] (rows 8-15 idle); bias / offset terms per group, too
+    float lift = 0x1p+100f, turn = 1.0f;  // what the warp's value scales and biases are multiplied by; what it changes by at the next tile
 #pragma unroll
     for (int i = 0; i < NBD; i++) oc[i][0] = oc[i][1] = oc[i][2] = oc[i][3] = 0.0f;
 #pragma unroll
     for (int g = 0; g < G; g++) side[g] = 0.0f;
 
-    if (s0 < s1) {
+    // Leaves a tile's scales in shared memory; a warp's threads hold the scales of the keys whose values it multiplies.  Value scales
+    // of at most 2^-QT_PLAIN are lifted, by as much for all the warp's keys so far, so that p * s keeps its bits as in the ring form.
+    // Above it does as it is: only p below 2^(QT_PLAIN - 14) fall among float16's subnormals, whose rounding (2^-25) is
+    // 2^(QT_PLAIN - 25) of the largest term.
+    auto keep_scales = [&](int to) {
+        float most = 0.0f;
 #pragma unroll
-        for (int g = 0; g < G; g++) sbuf[t * G + g] = nsb[g];
-    }
+        for (int g = 0; g < G; g++) most = fmaxf(most, fabsf(nsb[g].z));
+        const int k = qa_log2_ceil(__uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(most))));
+        const float up = fminf(k > -QT_PLAIN ? 1.0f : __uint_as_float((uint32_t)((int)QA_TOP - k + 127) << 23), lift);
+        turn = up * qa_inverse(lift);  // (at the first tile there is nothing to turn)
+        lift = up;
+#pragma unroll
+        for (int g = 0; g < G; g++) sbuf[(to * QA_TILE + t) * G + g] = make_float4(nsb[g].x, nsb[g].y, nsb[g].z * up, nsb[g].w * up);
+    };
+    if (s0 < s1) keep_scales(0);
     int buf = 0;
     for (int base = s0; base < s1; base += QA_TILE, buf ^= 1) {
         const int keys = min(QA_TILE, s1 - base);
@@ -924,13 +976,14 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
         if (c == 0) wred[1][warp][g8] = psum;
         __syncthreads();
         l = fmaf(l, corr, (wred[1][0][g8] + wred[1][1][g8]) + (wred[1][2][g8] + wred[1][3][g8]));
+        const float carry = corr * turn;
 #pragma unroll
         for (int i = 0; i < NBD; i++) {
-            oc[i][0] *= corr;
-            oc[i][1] *= corr;
+            oc[i][0] *= carry;
+            oc[i][1] *= carry;
         }
 #pragma unroll
-        for (int g = 0; g < G; g++) side[g] *= corr;
+        for (int g = 0; g < G; g++) side[g] *= carry;
         // ── values: two steps of 16 keys; the probabilities times the keys' value scales are the A fragments ──
 #pragma unroll
         for (int kk = 0; kk < 2; kk++) {
@@ -968,10 +1021,7 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
                 qa_mma(oc[nbd], pa0[nbd / NBD_PER_G], 0u, pa2[nbd / NBD_PER_G], 0u, b0, b1);
             }
         }
-        if (more) {
-#pragma unroll
-            for (int g = 0; g < G; g++) sbuf[((buf ^ 1) * QA_TILE + t) * G + g] = nsb[g];
-        }
+        if (more) keep_scales(buf ^ 1);
         __syncthreads();  // this tile's buffers are refilled from the next iteration on; wred is rewritten by the next tile
     }
 
@@ -982,12 +1032,13 @@ __global__ void __launch_bounds__(QA_THREADS, QT_BLOCKS) qattn_tile_kernel(QAttn
         side[g] += __shfl_xor_sync(0xFFFFFFFFu, side[g], 2);
     }
     float *wsum = reinterpret_cast<float *>(vbuf);  // [warp][head][D]
+    const float unlift = qa_inverse(lift);
     if (head) {
 #pragma unroll
         for (int nbd = 0; nbd < NBD; nbd++) {
             float *dst = wsum + ((warp * 8 + g8) * D) + 8 * nbd + 2 * c;
-            dst[0] = oc[nbd][0] + side[nbd / NBD_PER_G];
-            dst[1] = oc[nbd][1] + side[nbd / NBD_PER_G];
+            dst[0] = (oc[nbd][0] + side[nbd / NBD_PER_G]) * unlift;
+            dst[1] = (oc[nbd][1] + side[nbd / NBD_PER_G]) * unlift;
         }
     }
     __syncthreads();

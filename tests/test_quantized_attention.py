@@ -215,3 +215,108 @@ def test_kernel_at_the_edges_of_its_steps(D, bits, gs):
         k, v = make_cache(rng, 1, 1, S, D, oracle.BF16, gs, bits), make_cache(rng, 1, 1, S, D, oracle.BF16, gs, bits)
         q = oracle.from_f32(rng.standard_normal((1, 4, 1, D)).astype(np.float32), oracle.BF16)
         close(_run(nv, dev, q, k, v, oracle.BF16, gs, bits, 0.2, None, None), oat.dense(q, k, v, oracle.BF16, gs, bits, 0.2), TOL[oracle.BF16], f"s{S}")
+
+
+def _off(got, want):
+    return float(np.linalg.norm(got - want) / np.linalg.norm(want))
+
+
+# The queries times the scale and the probabilities times the value scales pass through float16 (half a unit: 2^-11), the latter
+# multiplying codes that are up to 5 times the values' deviation (groups of 64 values); the result is rounded to its type,
+# bfloat16's half unit being 2^-8, or 2^-25 at float16's subnormals.  Independent roundings of at most half a unit each: their root
+# mean squares (1 / sqrt 3 of it) add up as squares.  Scores of deviation d move by 2^-11 d / sqrt 3, and the probabilities by as
+# much relatively.  That is the mean over many results; over n of them the root mean square of errors even over half a unit has
+# a deviation of 0.45 / sqrt(n) of itself: five of these are allowed for.
+def _rounding(dtype, scores, want):
+    half = {oracle.BF16: 2.0 ** -8, oracle.F16: 2.0 ** -11}[dtype]
+    tiny = 2.0 ** -25 * np.sqrt(want.size) / np.linalg.norm(want) if dtype == oracle.F16 else 0.0
+    mean = np.sqrt((half ** 2 + tiny ** 2 + (5 * 2.0 ** -11) ** 2 + (5 * scores * 2.0 ** -11) ** 2) / 3)
+    return float(mean * (1 + 5 * 0.45 / np.sqrt(want.size)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("D,bits,gs", [(128, 8, 64), (64, 4, 32), (128, 4, 128)])
+def test_values_of_any_magnitude(dt, D, bits, gs):
+    """The error relative to the result's norm does not depend on the values' magnitude: both forms, peaked and flat scores,
+    and a cache whose first keys are a thousand times smaller or larger than the rest."""
+    import nuvec_b200 as nv
+    dev = nv.Device.shared(0)
+    dtype = DT[dt]
+    rng = np.random.default_rng(bits + D)
+    for S, L in ((700, 1), (700, 3), (9000, 1)):
+        k = make_cache(rng, 1, 2, S, D, dtype, gs, bits)
+        base = rng.standard_normal((2 * S, D)).astype(np.float32)
+        for std in (1e-4, 1e-3, 1e-2, 1.0, 1e2, "rising", "falling"):
+            factor = np.full((2, S, 1), 1e-3 if std == "rising" else 1.0 if std == "falling" else std, np.float32)
+            if isinstance(std, str):
+                factor[:, S // 3:] = 1.0 if std == "rising" else 1e-3
+            w = oracle.from_f32(base * factor.reshape(-1, 1), dtype)
+            v = tuple(a.reshape(1, 2, S, -1) for a in oracle.quantize(w, dtype, oracle.AFFINE, gs, bits))
+            for scores in (0.3, 3.0):
+                q = oracle.from_f32(rng.standard_normal((1, 4, L, D)).astype(np.float32), dtype)
+                got = _run(nv, dev, q, k, v, dtype, gs, bits, scores / np.sqrt(D), None, None)
+                want = oat.dense(q, k, v, dtype, gs, bits, scores / np.sqrt(D))
+                assert _off(got, want) <= _rounding(dtype, scores, want), (S, L, std, scores)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_one_row_over_long_caches(dt):
+    """The ring form at one query row: every number of query heads per key head, sinks, views of longer caches, several key heads
+    and batches, calls of different shapes back to back (they share scratch and arrival counters), very many splits."""
+    import nuvec_b200 as nv
+    dev = nv.Device.shared(0)
+    dtype = DT[dt]
+    rng = np.random.default_rng(29)
+    done = []
+    for D, bits, gs, B, Hq, Hkv, S, extra, sinks in ((128, 8, 64, 1, 1, 1, 4097, 0, False), (128, 4, 64, 1, 16, 8, 4500, 3, True), (64, 8, 32, 2, 8, 2, 5001, 60, True),
+                                                     (64, 4, 64, 3, 8, 1, 4111, 1, False), (128, 8, 128, 1, 16, 2, 6007, 9, True), (128, 8, 32, 2, 8, 8, 4099, 0, True),
+                                                     (64, 4, 32, 1, 8, 1, 65536, 0, True), (128, 4, 128, 1, 8, 2, 8191, 2, False)):
+        k, v = make_cache(rng, B, Hkv, S + extra, D, dtype, gs, bits), make_cache(rng, B, Hkv, S + extra, D, dtype, gs, bits)
+        q = oracle.from_f32(rng.standard_normal((B, Hq, 1, D)).astype(np.float32), dtype)
+        sink = oracle.from_f32(rng.standard_normal(Hq).astype(np.float32) * 4, dtype) if sinks else None
+        cut = lambda t: tuple(np.ascontiguousarray(a[:, :, :S]) for a in t)
+        want = oat.dense(q, cut(k), cut(v), dtype, gs, bits, 0.1, sink)
+        done.append(((q, k, v, gs, bits, sink, S), want, f"{dt} d{D} b{bits} gs{gs} B{B} hq{Hq} hkv{Hkv} s{S}"))
+    for (q, k, v, gs, bits, sink, S), want, name in done + done[::-1]:
+        got = _run(nv, dev, q, k, v, dtype, gs, bits, 0.1, sink, S)
+        assert _off(got, want) <= _rounding(dtype, 1.0, want), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_one_group_heads_read_nothing_behind_their_last_key(D, bits):
+    """With one group per head a row's scale is half a word, and the last key's word holds a value of the row behind it: NaN here."""
+    import nuvec_b200 as nv
+    dev = nv.Device.shared(0)
+    rng = np.random.default_rng(31)
+    dtype = oracle.BF16
+    for S, L, extra in ((37, 1, 3), (37, 3, 3), (16, 2, 1), (4097, 1, 2), (4113, 1, 1)):
+        k, v = make_cache(rng, 1, 2, S + extra, D, dtype, D, bits), make_cache(rng, 1, 2, S + extra, D, dtype, D, bits)
+        for t in (k, v):
+            for a in t[1:]:
+                a[:, :, S:] = 0x7FC0
+        q = oracle.from_f32(rng.standard_normal((1, 4, L, D)).astype(np.float32), dtype)
+        cut = lambda t: tuple(np.ascontiguousarray(a[:, :, :S]) for a in t)
+        want = oat.dense(q, cut(k), cut(v), dtype, D, bits, 0.1)
+        got = _run(nv, dev, q, k, v, dtype, D, bits, 0.1, None, S)
+        assert np.isfinite(got).all() and _off(got, want) <= _rounding(dtype, 1.0, want), (S, L)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_a_scale_that_is_no_number_stays_in_its_group(dt, bad):
+    import nuvec_b200 as nv
+    dev = nv.Device.shared(0)
+    rng = np.random.default_rng(37)
+    dtype = DT[dt]
+    for D, bits, gs, S, L in ((128, 8, 64, 300, 1), (128, 8, 64, 300, 3), (64, 4, 32, 4200, 1), (128, 4, 32, 40, 8)):
+        k, v = make_cache(rng, 1, 1, S, D, dtype, gs, bits), make_cache(rng, 1, 1, S, D, dtype, gs, bits)
+        q = oracle.from_f32(rng.standard_normal((1, 4, L, D)).astype(np.float32), dtype)
+        want = oat.dense(q, k, v, dtype, gs, bits, 0.1)[..., gs:]
+        v[1][0, 0, S // 2, 0] = oracle.from_f32(np.array([bad], np.float32), dtype)[0]
+        got = _run(nv, dev, q, k, v, dtype, gs, bits, 0.1, None, None)
+        assert not np.isfinite(got[..., :gs]).any() and _off(got[..., gs:], want) <= _rounding(dtype, 1.0, want), (D, bits, S, L)
