@@ -160,8 +160,25 @@ int array_init(PyObject *self, PyObject *args, PyObject *kw) {
         PyErr_SetString(PyExc_TypeError, "an array is initialized once");
         return -1;
     }
+    if (item_size(dtype) == 0) {
+        PyErr_Format(PyExc_KeyError, "%d is no dtype code", dtype);
+        return -1;
+    }
     a->shape = PySequence_Tuple(shape);
     if (!a->shape) return -1;
+    int64_t bytes = item_size(dtype);
+    for (Py_ssize_t i = 0; i < rank(a); i++) {
+        const int64_t d = dim(a, i);
+        if (d == -1 && PyErr_Occurred()) return -1;
+        if (d < 0) {
+            PyErr_Format(PyExc_ValueError, "an array of shape %R", a->shape);
+            return -1;
+        }
+        if (__builtin_mul_overflow(bytes, d, &bytes)) {
+            PyErr_Format(PyExc_OverflowError, "an array of shape %R", a->shape);
+            return -1;
+        }
+    }
     a->dtype = dtype;
     a->dev = Py_NewRef(dev);
     a->offset = offset;
