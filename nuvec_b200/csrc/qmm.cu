@@ -2,7 +2,6 @@
 // instantiations live in qmm_bf16.cu, qmm_f16.cu and qmm_fp.cu.
 #include "qmm_kernel.cuh"
 
-#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -94,37 +93,9 @@ int32_t launch_qmm(nvc_device *dev, const QmmParams &p) {
     if (p.rows == 0 || p.N == 0) return NVC_OK;
     const int64_t experts = p.offsets ? p.experts : 1;
     NVC_TRY(ensure_error_word(dev));
-    // The token tile (and whether blocks work in pairs): whichever plan is expected to finish soonest.  A fixed rule on the rows
-    // missed by up to 1.6 (219 x 4096 x 11008: 256 tokens 45 us, 128 tokens 27): how the tiles fill the last wave matters as
-    // much as a tile's own pace.  Experts' rows scatter around their average: the plan is weighed with the tiles that an
-    // average of six counts up to 2.25 standard deviations of a random routing away needs.  Grouped products do not pair: an
-    // expert's last token tile is rarely full and twice as many tiles balance better (32 experts x 2880 x 2880, 128 rows each:
-    // 105 us with pairs, 96 without).
-    static const struct { int bt; bool pair; } plans[] = {{32, false}, {64, false}, {128, false}, {160, false}, {192, false}, {256, false}, {256, true}};
-    const int sms = dev->prop.multiProcessorCount, kblocks = (int)(p.K / QMM_BK);
-    int bt = 32;
-    bool pair = false;
-    float best = INFINITY;
-    for (const auto &plan : plans) {
-        if (plan.pair && p.offsets) continue;
-        const int rows_per_tile = plan.pair ? 2 * QMM_BN : QMM_BN;
-        const int64_t n_tiles = (p.N + rows_per_tile - 1) / rows_per_tile;
-        float tok_tiles = (float)((p.rows + plan.bt - 1) / plan.bt);
-        if (p.offsets) {
-            const float per = (float)p.rows / (float)experts, sd = sqrtf(per);
-            tok_tiles = 0.0f;
-            for (int z = -5; z <= 5; z += 2) tok_tiles += ceilf(fmaxf(per + 0.45f * (float)z * sd, 0.0f) / (float)plan.bt) / 6.0f;
-            tok_tiles *= (float)experts;
-        }
-        const float tiles = fminf(tok_tiles * (float)n_tiles, 1e9f);
-        float ns;
-        make_schedule((int)(tiles + 0.5f), plan.pair ? sms / 2 : sms, kblocks, 4, plan.bt < p.rows ? plan.bt : (int)p.rows, qmm_block_ns(plan.bt, plan.pair, p.bits), &ns);
-        if (ns < best) {
-            best = ns;
-            bt = plan.bt;
-            pair = plan.pair;
-        }
-    }
+    const QmmPlan plan = qmm_plan(p.rows, p.offsets ? experts : 0, p.N, (int)(p.K / QMM_BK), p.bits, dev->prop.multiProcessorCount);
+    const int bt = plan.bt;
+    const bool pair = plan.pair;
     const int64_t token_tiles = (p.rows + bt - 1) / bt + (p.offsets ? experts : 0);  // grouped: at most, one partial tile per expert
     const bool affine = p.mode == NVC_AFFINE;
     QmmKernelParams kp{};

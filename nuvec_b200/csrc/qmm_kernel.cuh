@@ -43,6 +43,7 @@
 // gather, crates/nuvec-core/src/quantized.rs:679-719.
 #pragma once
 #include "qmm.cuh"
+#include "qmm_plan.h"
 #include "tcgen05.cuh"
 
 namespace nvc {
@@ -66,8 +67,6 @@ static __device__ long long g_qmm_timing[2][QT_ROLES][QT_SLOTS];
 #define QT_END(role, writer)
 #endif
 
-constexpr int QMM_BN = 128;  // weight rows per tile (UMMA M)
-constexpr int QMM_BK = 64;   // k-values per block: one 128-byte swizzle row of bfloat16
 constexpr int QMM_EPI_WARPS = 4, QMM_DQ_WARPS = 16, QMM_DQ_GROUPS = 4;  // dequantizers: groups of 4 warps
 constexpr uint32_t QMM_EPI_BARRIER = 9;  // named barrier of the epilogue warps (1 .. 8 belong to the stages)
 constexpr int QMM_WATCH_WARP = QMM_EPI_WARPS + 3 + QMM_DQ_WARPS;  // the warp that waits on behalf of the MMA warp
@@ -79,46 +78,6 @@ constexpr int QMM_TABLE_BYTES = 4112;        // the grouped products' tables: 2 
 constexpr int QMM_ITEMS = 64;                // a worker's first items, worked out once per block (see QmmWork)
 constexpr int QMM_ITEM_BYTES = QMM_ITEMS * 32;
 constexpr int QMM_EPI_STAGE_BYTES = 4 * 2048;  // epilogue: 32 tokens x 32 weight rows of bfloat16 per warp
-
-// The schedule.  Every worker (block, or pair of blocks) first takes `full_waves` whole tiles (tile = worker + wave *
-// workers).  The tiles left over (fewer than workers) are cut along K into `splits` parts of whole grains of k-blocks,
-// dealt over the workers in `tail_rounds` rounds, so that the last wave -- or a product with fewer tiles than
-// multiprocessors -- still keeps every multiprocessor busy.  Parts leave float32 partial tiles in scratch; the block that
-// arrives last adds them in part order and writes the result.
-struct Schedule {
-    int32_t full_waves, tail_tiles, splits, tail_rounds;
-};
-// What the plan is weighed with, in ns: a worker's pace per 64-k block with tiles of BT tokens, and the price of cutting a tile
-// (a part's way through scratch and the arrival, then the addition, which reads every part at about 100 bytes per ns).
-// Measured over 16 shapes between 24 and 2048 rows: up to 128 tokens the dequantization sets the pace, from 256 on the MMAs;
-// 160 and 192 have smaller stages.  More bits per code take longer to unpack.
-__host__ __device__ constexpr float qmm_block_ns(int bt, bool pair, int bits) {
-    return (bt <= 64 ? 220.0f : bt <= 128 ? 255.0f : bt <= 160 ? 315.0f : bt <= 192 ? 340.0f : pair ? 420.0f : 450.0f) *
-           (bits == 2 || bits == 4 ? 1.0f : bt <= 192 ? 1.15f : 1.08f);
-}
-// tokens: of a tile, at most.  *ns: the plan's expected duration.
-__host__ __device__ inline Schedule make_schedule(int tiles, int workers, int kblocks, int grain, int tokens, float block_ns, float *ns) {
-    Schedule c{tiles / workers, tiles % workers, 1, 1};
-    const int grains = (kblocks + grain - 1) / grain;
-    float tail = 0.0f;
-    if (c.tail_tiles > 0) {
-        // Parts per tile: whatever makes the left-over tiles finish soonest when the parts are dealt over the workers in one or
-        // two rounds; at least two grains of k-blocks per part, at most 16 parts.
-        tail = (float)kblocks * block_ns;
-        for (int s = 2; s <= 16 && s <= grains / 2; s++) {
-            const int rounds = (c.tail_tiles * s + workers - 1) / workers;
-            if (rounds > 2) break;
-            const float cost = (float)(rounds * ((grains + s - 1) / s) * grain) * block_ns + 2000.0f + 5.0f * (float)(rounds * s * tokens);
-            if (cost < tail) {
-                tail = cost;
-                c.splits = s;
-            }
-        }
-        c.tail_rounds = (c.tail_tiles * c.splits + workers - 1) / workers;
-    }
-    *ns = (float)c.full_waves * (float)kblocks * block_ns + tail;
-    return c;
-}
 
 struct QmmKernelParams {
     const uint8_t *scales, *biases;   // [weight rows, K / gs]: 16-bit values, or one byte each (mxfp4 / mxfp8 / nvfp4, no biases)

@@ -8,6 +8,7 @@ import pytest
 import nuvec_b200 as nv
 import oracle
 from cuda_backend import CudaBackend, host
+from test_qmm_plan import SHAPES
 
 pytestmark = pytest.mark.gpu
 
@@ -113,7 +114,7 @@ def same(got, want, dt):
 @pytest.mark.parametrize("fmt", FORMATS)
 def test_many_rows_at_the_tiles_edges(be, fmt):
     """Around every token tile, one to 21 k-blocks (an odd number leaves half a stage), rows of scales on no boundary, N no
-    multiple of 128, tiles cut along K, and (the last two) pairs of blocks whose last tile has one block's rows only."""
+    multiple of 128, tiles cut along K, pairs of blocks."""
     mode, bits, gs, dt = fmt
     rng = np.random.default_rng(bits + gs)
     for M, N, K in ((9, 128, 128), (32, 130, 192), (33, 8, 1344), (64, 136, 4224), (65, 257, 128), (129, 260, 320), (160, 128, 1344), (161, 390, 576),
@@ -124,6 +125,18 @@ def test_many_rows_at_the_tiles_edges(be, fmt):
         x, ks = unit(rng, M, K, dt)
         got = be.quantized_matmul(x, c, s, b, CODE[dt], mode, gs, bits, True)
         assert same(got, dense[:, ks].T, dt), (M, N, K)
+
+
+@pytest.mark.parametrize("fmt,shape", [(f, s) for f in FORMATS for s in SHAPES if s[2] % f[2] == 0 and s[0] * s[1] * s[2] < 10 ** 10])
+def test_many_rows_in_every_plan(be, fmt, shape):
+    """Every token tile, single blocks and pairs (198 x 9490: the last pair has weight rows for its first block only)."""
+    mode, bits, gs, dt = fmt
+    M, N, K = shape
+    assert nv.Device.shared(0).info()["multiprocessors"] == 148  # (the plans of these shapes, see test_qmm_plan.py)
+    rng = np.random.default_rng(bits + gs + M)
+    c, s, b, dense = packed(rng, N, K, fmt)
+    x, ks = unit(rng, M, K, dt)
+    assert same(be.quantized_matmul(x, c, s, b, CODE[dt], mode, gs, bits, True), dense[:, ks].T, dt)
 
 
 @pytest.mark.parametrize("fmt", [FORMATS[0], FORMATS[4], *FORMATS[-4:]])
