@@ -1083,11 +1083,20 @@ static int32_t qattn_combine(nvc_device *dev, const QAttnParams &p) {
 }
 
 // The form of a call.  CUDA cores: float32 and 3-bit codes (NUVEC_QATTN_MMA=0: everything).  The ring form reads a row's scales
-// as one word or two.  The tile form takes what is not so aligned, and one query row over up to 4096 keys and 4 MiB of key
-// codes: there the two are within 1.7 us of one another either way (one batch of 8 key heads of 128, 8 bits: 1000 keys 7.2 us by
-// ring, 7.5 by tiles, 4000 keys 9.9 and 11.5, 8000 keys 13.1 and 16.7; four batches of 4 key heads, 1000 keys, 4 bits: 8.8 and
-// 7.4), which is not worth other bits: through six layers of a decode step another rounding of the attention moves the outputs
-// by 1.7e-2, relatively.
+// as one word or two.  The tile form takes what is not so aligned, and one query row over few keys.
+//
+// Where the line lies: a block of the tile form takes a tile of 128 keys from beginning to end, with nothing to overlap it, and
+// its merge is a launch that walks a head's splits one after another; the ring form's warps need a few steps each to fill their
+// rings, and its merge is a round trip through global memory.  So the bytes per multiprocessor decide, and the splits per head.
+// Measured over 1 to 8 batches x 1 to 8 key heads of 128 x 64 to 8000 keys, four query heads each, us by tiles over us by ring:
+//     codes of the keys    up to 2 MiB     4 MiB           8 MiB           16 MiB
+//     4 bits               0.77 .. 1.19    1.09 .. 1.12    1.41 .. 1.52    1.54 .. 1.62
+//     8 bits               0.92 .. 1.25    0.98 .. 1.19    1.31 .. 1.34    1.68 .. 1.70
+//     one to eight heads of 8000 keys (63 splits): 1.05 .. 1.45
+// Up to 4 MiB and 32 splits neither form is ahead of the other by more than a quarter, 1.9 us a call; beyond, the ring form
+// always is.  (Up to 128 keys are the exception: the ring form needs no merge there, 3.4 us against 6.2.)  Within the range the
+// tile form stays for its results: both forms are equally exact (4 to 6e-4 before the rounding to bfloat16), but another rounding
+// of the attention moves the outputs of three to six layers of a decode step by 1.1 to 1.7e-2, and gained those steps 0.2 to 1.9 %.
 enum QaForm { QA_CUDA, QA_TILES, QA_RING };
 static QaForm qattn_form(int dtype, int bits, int64_t groups, std::initializer_list<const void *> scales, const void *q, const void *out, int64_t L, int64_t S,
                          int64_t code_bytes) {

@@ -149,9 +149,10 @@ extern "C" int32_t nvc_quantized_matmul(nvc_device *dev, const nvc_quant *q, int
         }
         return NVC_OK;
     }
-    // Many rows of a bit width only the few-row kernel decodes fast (3 and 6 bits): eight rows at a
-    // time through it.  The weights are streamed once per eight rows (from L2 when they fit), which
-    // is far from the tensor-core kernel but two orders of magnitude ahead of the generic one.
+    // Many rows of a shape that the tensor-core kernel does not take and the few-row kernel does (K a
+    // multiple of 32, not of 64): eight rows at a time through it.  The weights are streamed once per
+    // eight rows (from L2 when they fit), which is far from the tensor-core kernel but two orders of
+    // magnitude ahead of the generic one.
     if (M > 8 && q->mode == NVC_AFFINE &&
         qmv_affine_eligible(q->mode, q->group_size, q->bits, dtype, transpose, 8, N, K, x, ldx, 0, w, 0)) {
         const size_t esz = dtype_size(dtype);

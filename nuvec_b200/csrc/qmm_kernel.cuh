@@ -393,7 +393,7 @@ template <int BT, int GRAIN, bool PAIR> struct QmmWork {
 // PAIR: two blocks of a cluster (cta_group::2) share a tile of 2 x 128 weight rows x BT tokens; each keeps half of the
 // tokens' activations in its shared memory and its own rows' weights and accumulator in its tensor memory.  An MMA of 128
 // rows reads its token operand from shared memory at half of that memory's bandwidth, and writing the stages takes the other
-// half: at 192 and 256 tokens, where the MMAs set the pace, single blocks took 164 us for 2048 x 12288 x 4096, pairs 147.
+// half: at 256 tokens, where the MMAs set the pace, single blocks take 158 us for 2048 x 12288 x 4096, pairs 150 (8 bits: 173, 160).
 template <int BITS, int BT, int MODE, bool PAIR> struct QmmShape {
     static constexpr int SUB = BT <= 128 || PAIR ? 2 : 1;
     static constexpr int KPS = SUB == 2 ? 2 : BITS == 2 ? 8 : BITS <= 4 ? 4 : 2;  // 64-k blocks per slab
