@@ -281,7 +281,8 @@ __device__ __forceinline__ float qa_exp2(float x) {  // 2 to the x, relative err
 // relative error 0.86 at 16K keys, 8 bits.)  It is a score plus a whole number: the key that set it has a power of two for its p,
 // and so an exact p * s (whole reference points: peaked scores 8e-4 off instead of 5e-4).
 constexpr float QA_SLACK = 3.0f, QA_TOP = 15.0f;  // room above the largest score when the reference moves; log2 of the largest p * s
-constexpr int QA_K_MIN = -26, QA_K_MAX = 55;      // scales outside are taken as these: sums of 2^(QA_TOP - k) * p stay in float32's range
+// Scales outside are taken as these: 2^(QA_TOP - k) * p, its sums, and its products with biases of up to 2^86 stay in float32's range.
+constexpr int QA_K_MIN = -26, QA_K_MAX = 55;
 __device__ __forceinline__ int qa_log2_ceil(float s) {  // of s >= 0, in [QA_K_MIN, QA_K_MAX]
     const uint32_t u = __float_as_uint(s);
     return min(max((int)(u >> 23) - 127 + ((u & 0x7FFFFFu) != 0u ? 1 : 0), QA_K_MIN), QA_K_MAX);
